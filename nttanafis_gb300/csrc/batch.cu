@@ -386,10 +386,15 @@ uint8_t ntt_batch_run_device(ntt_batch* b, const ntt_request* reqs, size_t count
         if (!cuda_ok(cudaMemsetAsync(reqs[i].dst, 0, ((size_t)reqs[i].a_len + reqs[i].b_len) * 8, st), "zero product"))
             return 0;
     if (members.empty() && splits.empty()) return 1;
-    // Group by class: kind, schoolbook, transform length, primes, sign, square.
-    std::sort(members.begin(), members.end(), [](const Member& x, const Member& y) {
-        return std::make_tuple(x.g.conv, x.g.schoolbook, x.g.log_t, x.g.np, x.g.sign, x.square, x.index) <
-               std::make_tuple(y.g.conv, y.g.schoolbook, y.g.log_t, y.g.np, y.g.sign, y.square, y.index);
+    // Group by class: kind, schoolbook, transform length, primes, sign, square. Two members
+    // of one length and prime count may still differ in their prime class (at 2^22 and 2^23
+    // points, five lazy or five wide primes by their shorter operands).
+    const auto class_of = [](const Member& m) {
+        return std::make_tuple(m.g.conv, m.g.schoolbook, m.g.log_t, m.g.np, m.g.wide, m.g.sign, m.square);
+    };
+    std::sort(members.begin(), members.end(), [&](const Member& x, const Member& y) {
+        const auto cx = class_of(x), cy = class_of(y);
+        return cx != cy ? cx < cy : x.index < y.index;
     });
     if (!b->arena.ensure(std::max<u64>(arena_bytes, 256)) || !b->desc.ensure(members.size() * sizeof(ProductDesc)))
         return 0;
@@ -451,10 +456,7 @@ uint8_t ntt_batch_run_device(ntt_batch* b, const ntt_request* reqs, size_t count
     while (k < members.size()) {
         const Geom& g0 = members[k].g;
         size_t end = k + 1;
-        while (end < members.size() && end - k < kMaxLaunchMembers && members[end].g.conv == g0.conv &&
-               members[end].g.schoolbook == g0.schoolbook && members[end].g.log_t == g0.log_t &&
-               members[end].g.np == g0.np && members[end].g.sign == g0.sign &&
-               members[end].square == members[k].square)
+        while (end < members.size() && end - k < kMaxLaunchMembers && class_of(members[end]) == class_of(members[k]))
             ++end;
         if (g0.conv && g0.schoolbook) {
             for (size_t i = k; i < end; ++i) {

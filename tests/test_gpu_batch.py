@@ -182,3 +182,35 @@ def test_unbalanced_members_run_as_block_splits(gpu):
     assert batch.split_members == 9  # three split members per run
     assert batch.status() == 0
     batch.close()
+
+
+@pytest.mark.parametrize("lazy_first", [True, False])
+def test_members_of_both_prime_classes_at_one_length(gpu, lazy_first):
+    """Two products of 2^22 points on five primes each, one on the lazy primes (a
+    shorter operand of 2^20 limbs), one on the wide ones (2^21 limbs, whose largest
+    coefficients the lazy set does not hold): two classes of one batch."""
+    import torch
+
+    lengths = [(3 << 20, 1 << 20), (1 << 21, 1 << 21)]
+    if not lazy_first:
+        lengths.reverse()
+    plans = [gpu.MulPlan.new(la, lb) for la, lb in lengths]
+    assert {p.log_transform for p in plans} == {22} and {p.primes for p in plans} == {5}
+    reqs = []
+    for la, lb in lengths:
+        a, b = (torch.full((n,), -1, dtype=torch.int64, device="cuda") for n in (la, lb))
+        reqs.append(gpu.Request(torch.zeros(la + lb, dtype=torch.int64, device="cuda"), a, b))
+    batch = gpu.GpuBatch()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(2):
+        assert batch.run(reqs, stream), gpu.last_error()
+    stream.synchronize()
+    assert batch.status() == 0
+    for (la, lb), r in zip(lengths, reqs):  # (B^la - 1)(B^lb - 1)
+        want = torch.zeros(la + lb, dtype=torch.int64, device="cuda")
+        want[0] = 1
+        want[min(la, lb):] = -1
+        want[max(la, lb)] = -2
+        assert torch.equal(r.dst, want), (la, lb)
+    batch.close()
