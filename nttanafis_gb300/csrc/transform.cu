@@ -540,8 +540,9 @@ __global__ void __launch_bounds__(kCol4Threads, kCol4LogG == 2 ? 2 : 1)
 }
 
 // Persistent form of k_inv_cols4, for residues that start on a 16-byte boundary (a
-// caller's scratch need not; k_inv_cols4 reads those): one CTA per SM loops over the (column group, prime, member) items. Once an item's second pass holds
-// its points in registers, the shared buffer is free, and 16-byte cp.async copies
+// caller's scratch need not; k_inv_cols4 reads those): one CTA per SM loops over the
+// (column group, prime, member) items. Once an item's second pass holds its points in
+// registers, the shared buffer is free, and 16-byte cp.async copies
 // bring the next item's residues into it while that pass computes and stores, so
 // that the loads of one item overlap the butterflies of the one before. The copies
 // land in a raw layout, row 64b + k of the 8 columns at word 520b + 8k: the first
@@ -1027,8 +1028,10 @@ static cudaError_t inv_cols_cut(const TransformArgs& g, cudaStream_t st, bool in
             const cudaError_t e = opt_in(p, col_carveout(L));
             return e == cudaSuccess ? opt_in(k, col_carveout(L)) : e;
         }
-        // members of a batch start on 256-byte boundaries
-        if (!g.batch && (reinterpret_cast<uintptr_t>(g.spec) & 15) != 0)
+        // members of a batch start on 256-byte boundaries, blocks of a split product a
+        // multiple of 256 bytes after the shorter operand's spectrum in the caller's scratch
+        const u32* first = g.batch ? g.shared_spec : g.spec;
+        if ((reinterpret_cast<uintptr_t>(first) & 15) != 0)
             return launch_dependent(k, grid, dim3(kCol4Threads), col4_smem(false), st, g);
         const unsigned items = grid.x * grid.y * grid.z;
         return launch_dependent(p, dim3(std::min(items, (unsigned)sm_count())), dim3(kCol4Threads), col4p_smem(g.np),

@@ -130,3 +130,22 @@ def test_wide_plan_call_with_scratch_off_the_16_byte_boundary(gpu):
         assert plan.mul_device(dst, a, b, scratch, torch.cuda.current_stream()), gpu.last_error()
         torch.cuda.synchronize()
         assert torch.equal(dst, want)
+
+
+def test_wide_block_split_with_scratch_off_the_16_byte_boundary(gpu):
+    # blocks of 2^24 points, whose residues lie in the caller's scratch
+    import torch
+
+    la, lb = 40_000_000, 2_000_000
+    plan = gpu.MulPlan.new(la, lb)
+    assert plan.blocks > 1 and plan.log_transform == 24
+    scratch = torch.zeros(plan.scratch_len() + 1, dtype=torch.int64, device="cuda")[1:]
+    assert scratch.data_ptr() % 16 == 8
+    a, b = (torch.full((n,), -1, dtype=torch.int64, device="cuda") for n in (la, lb))
+    dst = torch.zeros(la + lb, dtype=torch.int64, device="cuda")
+    for x, y in ((a, b), (b, a)):
+        dst.zero_()
+        plan = gpu.MulPlan.new(x.numel(), y.numel())
+        assert plan.mul_device(dst, x, y, scratch, torch.cuda.current_stream()), gpu.last_error()
+        torch.cuda.synchronize()
+        assert torch.equal(dst, torch.from_numpy(all_ones_product(la, lb).view(np.int64)).cuda())
