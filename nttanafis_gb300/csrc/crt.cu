@@ -112,9 +112,13 @@ __global__ void __launch_bounds__(kCrtThreads, WIDE ? 6 : 5) k_crt_mul(const u32
                                                           u64 conv_len, u64 out_len, u64* __restrict__ dst,
                                                           u32* __restrict__ flags,
                                                           const __grid_constant__ CrtParams cp,
-                                                          const ProductDesc* __restrict__ batch,
+                                                          const ProductDesc* batch,
                                                           u32* __restrict__ status) {
     constexpr int L = crt_limb_words(NP);
+    // the residues and cleared flags of the transform before it, and in a block split the
+    // descriptors (no __restrict__: they are not constant while the kernel waits)
+    wait_prior_grid();
+    release_dependents();  // the next product's first kernel
     if (batch) {  // member blockIdx.y of a batch: grid.x covers its largest member
         const ProductDesc& d = batch[blockIdx.y];
         resid = d.spec;
@@ -123,8 +127,6 @@ __global__ void __launch_bounds__(kCrtThreads, WIDE ? 6 : 5) k_crt_mul(const u32
         dst = d.dst;
         flags = reinterpret_cast<u32*>(d.agg);
     }
-    wait_prior_grid();  // the residues and cleared flags of the transform before it
-    release_dependents();  // the next product's first kernel
     // Tiles are numbered in the order CTAs start, so a tile only ever waits for
     // tiles whose CTAs are already running.
     __shared__ u32 s_tile;

@@ -296,9 +296,10 @@ void set_last_error(const std::string& message);
 // CTAs are running. Every kernel of a single call is launched so, the first one too: the
 // launch then overlaps the end of whatever ran before it, the product before it above
 // all (whose last kernel releases it early). The first kernel of a batch class is not
-// (first_dependent). Of the members' passes, the row and inverse column passes read the
-// descriptors before they wait, so the column pass waits before it releases them. Both
-// device calls are no-ops for a kernel launched without the attribute.
+// (first_dependent): its descriptors are copied in ahead of it, so the row and inverse
+// column passes of the class read them before they wait. Those of a block split come from
+// a kernel of the sequence (k_split_descs), and every pass reads them after its wait.
+// Both device calls are no-ops for a kernel launched without the attribute.
 // What an earlier kernel wrote is read with __ldcg, not through the read-only path
 // (__ldg): it may be written while the kernel that reads it is already running.
 // The first kernel launched so, against normally, per product back to back: 48 x 48

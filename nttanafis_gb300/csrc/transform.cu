@@ -78,7 +78,7 @@ template <class A, bool SIGNED, int LOG_R, bool CUT, bool CHECK = SIGNED>
 __global__ void __launch_bounds__(kThreads) k_fwd_cols(const __grid_constant__ TransformArgs g) {
     extern __shared__ u32 sm[];
     using M = ColumnMap<LOG_R>;
-    if (g.batch) wait_prior_grid();  // the descriptors, which the dependents read before they wait
+    if (g.batch) wait_prior_grid();  // descriptors that the kernel before may write
     release_dependents();
     constexpr int B = M::SWEEPS < 8 ? M::SWEEPS : 8;  // sweeps per batch; B*RS is a multiple of 32
     static_assert(M::SWEEPS % B == 0 && (B * M::RS) % 32 == 0, "column batches");
@@ -240,7 +240,7 @@ template <class A, bool SIGNED, int LOG_R, bool CUT, bool CHECK = SIGNED>
 __global__ void __launch_bounds__(Columns<LOG_R>::NT, Columns<LOG_R>::MINB)
     k_fwd_cols2(const __grid_constant__ TransformArgs g) {
     extern __shared__ u32 sm[];
-    if (g.batch) wait_prior_grid();  // the descriptors, which the dependents read before they wait
+    if (g.batch) wait_prior_grid();  // descriptors that the kernel before may write
     release_dependents();
     using K = Columns<LOG_R>;
     constexpr int G = K::G, EA = K::EA, EB = K::EB;
@@ -329,9 +329,10 @@ __global__ void __launch_bounds__(Columns<LOG_R>::NT, Columns<LOG_R>::MINB)
     constexpr int G = K::G, EA = K::EA, EB = K::EB;
     const int prime = blockIdx.y;
     const PrimeParams& pp = g.ps.pr[prime];
+    release_dependents();
+    if (g.shared_spec) wait_prior_grid();  // descriptors that a kernel of the sequence wrote
     const Member m = member_of(g, blockIdx.z, false);
     const int octs = CUT ? octants_of(m.conv_len, g.log_t) : kOctants;
-    release_dependents();
     const int log_c = g.log_c;
     const int c = threadIdx.x & (G - 1), blk = threadIdx.x >> K::LOG_G;
     wait_prior_grid();  // the row pass's output
@@ -412,7 +413,7 @@ template <class A, bool SIGNED, bool CUT, bool CHECK = SIGNED>
 __global__ void __launch_bounds__(kCol4Threads, kCol4LogG == 2 ? 2 : 1)
     k_fwd_cols4(const __grid_constant__ TransformArgs g) {
     extern __shared__ u32 sm[];
-    if (g.batch) wait_prior_grid();  // the descriptors, which the dependents read before they wait
+    if (g.batch) wait_prior_grid();  // descriptors that the kernel before may write
     release_dependents();
     constexpr int G = kCol4G, LOG_G = kCol4LogG, VS = kCol4Vs, E = 64;
     // grid.x runs over (column group, prime) with the prime fastest, so the np CTAs
@@ -499,9 +500,10 @@ __global__ void __launch_bounds__(kCol4Threads, kCol4LogG == 2 ? 2 : 1)
     constexpr int G = kCol4G, LOG_G = kCol4LogG, VS = kCol4Vs, E = 64;
     const int prime = blockIdx.y;
     const PrimeParams& pp = g.ps.pr[prime];
+    release_dependents();
+    if (g.shared_spec) wait_prior_grid();  // descriptors that a kernel of the sequence wrote
     const Member m = member_of(g, blockIdx.z, false);
     const int octs = CUT ? octants_of(m.conv_len, g.log_t) : kOctants;
-    release_dependents();
     const int log_c = g.log_c;
     const int c = threadIdx.x & (G - 1), blk = threadIdx.x >> LOG_G;
     uint2* tw = reinterpret_cast<uint2*>(sm + G * VS);
@@ -681,13 +683,15 @@ __global__ void __launch_bounds__(row_threads(LOG_C)) k_rows(const __grid_consta
     const int prime = blockIdx.y;
     const int row0 = blockIdx.x << LOG_RPC;
     const PrimeParams& pp = g.ps.pr[prime];
-    const Member m = member_of(g, blockIdx.z, NV == 1);
+    // Blocks of a split product (kRowPre): descriptors that a kernel of the sequence wrote,
+    // read after the wait. Their transforms are filled (no cut).
+    Member m;
+    if constexpr (MODE != kRowPre) m = member_of(g, blockIdx.z, NV == 1);
     if constexpr (!kRowsReleaseLate<LOG_C>) release_dependents();
     // rows of octants that the member's coefficients do not need (a CTA whose first row
     // is needed may hold unneeded ones as well: what it makes of them is not read)
-    if (g.cut && row0 >= octants_of(m.conv_len, g.log_t) << (g.log_r - 3)) return;
-    u32* ra = m.spec + ((size_t)prime << g.log_t) + ((size_t)row0 << LOG_C);
-    const u32* rb = m.spec + ((size_t)(g.np + prime) << g.log_t) + ((size_t)row0 << LOG_C);
+    if constexpr (MODE != kRowPre)
+        if (g.cut && row0 >= octants_of(m.conv_len, g.log_t) << (g.log_r - 3)) return;
     // the stored spectrum of the rows (kRowFwd writes it, kRowPre multiplies by it)
     u32* rs = g.shared_spec + ((size_t)prime << g.log_t) + ((size_t)row0 << LOG_C);
     // The rows' inverse four-step factors: RPC x 64 low-digit entries, RPC x C/64 high.
@@ -701,6 +705,9 @@ __global__ void __launch_bounds__(row_threads(LOG_C)) k_rows(const __grid_consta
     }
     wait_prior_grid();  // the column pass's output
     if constexpr (kRowsReleaseLate<LOG_C>) release_dependents();
+    if constexpr (MODE == kRowPre) m = member_of(g, blockIdx.z, true);
+    u32* ra = m.spec + ((size_t)prime << g.log_t) + ((size_t)row0 << LOG_C);
+    const u32* rb = m.spec + ((size_t)(g.np + prime) << g.log_t) + ((size_t)row0 << LOG_C);
     // First forward pass: global -> shared. Block gg of a row holds points gg + k * HQ.
     {
         constexpr int LOG_HQ = LOG_C - RB;
@@ -803,9 +810,10 @@ __global__ void __launch_bounds__(kThreads) k_inv_cols(const __grid_constant__ T
     static_assert(M::SWEEPS % B == 0 && (B * M::RS) % 32 == 0, "column batches");
     const int prime = blockIdx.y;
     const PrimeParams& pp = g.ps.pr[prime];
+    release_dependents();
+    if (g.shared_spec) wait_prior_grid();  // descriptors that a kernel of the sequence wrote
     const Member m = member_of(g, blockIdx.z, false);
     const int octs = CUT ? octants_of(m.conv_len, g.log_t) : kOctants;
-    release_dependents();
     const u64 step = (u64)M::RS << g.log_c;
     u32* const base = m.spec + ((size_t)prime << g.log_t) + ((u64)M::row0() << g.log_c) +
                       (blockIdx.x << M::LOG_G) + M::col();

@@ -86,3 +86,41 @@ def test_dependent_products_captured_in_a_graph(gpu):
     del graph
     ws.close()
     cws.close()
+
+
+# block splits on one-CTA blocks (2^11..2^13 points), on four-step ones and in more than
+# one chunk of blocks, either operand the longer one, beside unsplit products
+LONGEST = (30_000_000, 3000)
+SPLITS = [(1 << 20, 1000), (4096, 4096), (3001, 1 << 20), (600000, 20000), (200000, 1000), (1 << 20, 100003),
+          (65536, 65536), LONGEST, (1 << 20, 1000), (100003, 600000), (700, 600), (1 << 18, 300)]
+
+
+def test_dependent_block_splits_on_one_stream(gpu):
+    import torch
+
+    plans = [gpu.MulPlan.new(la, lb) for la, lb in SPLITS]
+    split = {p.log_transform for p in plans if p.blocks}
+    assert min(split) < 13 < max(split)
+    longest = gpu.MulPlan.new(*LONGEST)
+    assert longest.blocks * (20 << longest.log_transform) > 512 << 20  # above one chunk's arena
+    pool = torch.from_numpy(operand(LONGEST[0], 17).view(np.int64)).cuda()
+    pairs = [(pool[:la], pool[-lb:]) for la, lb in SPLITS]
+    outs = [[torch.full((la + lb,), -1, dtype=torch.int64, device="cuda") for la, lb in SPLITS] for _ in range(4)]
+    scratch = torch.full((max(p.scratch_len() for p in plans),), 0x5A5A5A5A5A5A5A5A, dtype=torch.int64, device="cuda")
+    ws = gpu.GpuMulWorkspace()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for dsts in outs[:2]:  # the workspace's scratch, which every product overwrites
+        for dst, (a, b) in zip(dsts, pairs):
+            assert ws.mul_device(dst, a, b, stream), gpu.last_error()
+    for dsts in outs[2:]:  # a caller's scratch
+        for dst, (a, b), plan in zip(dsts, pairs, plans):
+            assert plan.mul_device(dst, a, b, scratch, stream), gpu.last_error()
+    stream.synchronize()
+    assert ws.status() == 0
+    for k, (a, b) in enumerate(pairs):
+        x, y = (v.cpu().numpy().view(np.uint64) for v in (a, b))
+        want = torch.from_numpy(oracle.mul(x, y, 16).view(np.int64)).cuda()
+        for dsts in outs:
+            assert torch.equal(dsts[k], want), SPLITS[k]
+    ws.close()
