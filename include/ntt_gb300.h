@@ -301,15 +301,18 @@ uint8_t ntt_crt_pair_combine_device(uint64_t first, uint64_t second, int64_t* d_
                                     const uint64_t* d_second, size_t n, void* stream);
 
 /* Four-step split T = R * C of the lazy transform lengths 2^14..2^23, process-wide:
- * ntt_split_set makes R = 2^log_r for transforms of 2^log_t points (0 restores the
- * default, min(floor(log_t / 2), 10), which ntt_split_get reports) and returns the
- * previous log_r, or -1 when log_t has no choice of split or log_r is outside the range
- * that ntt_split_range reports (columns 2^6..2^11, rows 2^7..2^13). By default a product
- * enqueued alone takes max(log_t - 10, 6) up to 2^18 points and log_t - 12 at 2^20 and
- * 2^21 instead. ntt_split_get
- * returns the log_r in use (0 for lengths without a four-step split). The split changes
- * speed, never results.
- * ntt_tune_splits times every split of each length in [min_log_t, max_log_t] on
+ * ntt_split_set makes R = 2^log_r for transforms of 2^log_t points. 0 restores the
+ * default, and so does the default's own value, min(floor(log_t / 2), 10): setting back
+ * what a call returned restores what was there before it. It returns the previous log_r,
+ * or -1 when log_t has no choice of split or log_r is outside the range that
+ * ntt_split_range reports (columns 2^6..2^11, rows 2^7..2^13). While no split is set, a
+ * product or convolution enqueued alone takes another one than batch members do at some
+ * lengths: max(log_t - 10, 6) up to 2^18 points and log_t - 12 at 2^20 and 2^21.
+ * ntt_split_get returns the log_r of batch members, ntt_split_lone that of products
+ * enqueued alone (on the lazy primes), and ntt_split_chosen the one that was set (0: none,
+ * the defaults hold); each 0 for lengths without a choice. The split changes speed, never
+ * results.
+ * ntt_tune_splits times every settable split of each length in [min_log_t, max_log_t] on
  * products that fill the transform on the lazy primes (balanced up to 2^21 points,
  * a 2^19-limb shorter operand above; `reps` products per timing, best of two) on
  * `stream` and keeps the fastest when it beats the default by 2%; it
@@ -325,6 +328,8 @@ uint8_t ntt_crt_pair_combine_device(uint64_t first, uint64_t second, int64_t* d_
 uint64_t ntt_school_set(uint64_t max_products);
 int ntt_split_set(int log_t, int log_r);
 int ntt_split_get(int log_t);
+int ntt_split_chosen(int log_t);
+int ntt_split_lone(int log_t);
 int ntt_split_range(int log_t, int* lo, int* hi);
 uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream);
 

@@ -115,6 +115,8 @@ _SIGNATURES = [
     ("ntt_school_set", ctypes.c_uint64, [ctypes.c_uint64]),
     ("ntt_split_set", ctypes.c_int, [ctypes.c_int, ctypes.c_int]),
     ("ntt_split_get", ctypes.c_int, [ctypes.c_int]),
+    ("ntt_split_chosen", ctypes.c_int, [ctypes.c_int]),
+    ("ntt_split_lone", ctypes.c_int, [ctypes.c_int]),
     ("ntt_split_range", ctypes.c_int, [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
     ("ntt_tune_splits", ctypes.c_uint8, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]),
     ("ntt_field_check", ctypes.c_int, [ctypes.c_uint64]),
@@ -206,12 +208,20 @@ def split_range(log_t: int) -> Optional[tuple[int, int]]:
 
 
 def get_split(log_t: int) -> int:
-    """log2 R of the four-step split in use for 2^log_t points (0: no four-step form)."""
+    """log2 R of the four-step split of batch members of 2^log_t points (0: no four-step
+    form). Products enqueued alone take lone_split's while no split is set."""
     return int(library().ntt_split_get(log_t))
 
 
+def lone_split(log_t: int) -> int:
+    """log2 R of the four-step split that a product of 2^log_t points enqueued alone runs
+    on the lazy primes (0: no choice of split)."""
+    return int(library().ntt_split_lone(log_t))
+
+
 def set_split(log_t: int, log_r: int) -> int:
-    """Sets log2 R for 2^log_t points (0: the default); returns the previous one."""
+    """Sets log2 R for 2^log_t points (0, or what get_split reports untouched: the
+    default); returns the previous one, which set again restores what was there."""
     prev = int(library().ntt_split_set(log_t, log_r))
     if prev < 0:
         raise ValueError(f"no split 2^{log_r} for transforms of 2^{log_t} points")
@@ -227,23 +237,24 @@ def tune_splits(min_log_t: int = 14, max_log_t: int = 23, reps: int = 5, stream=
 
 
 def save_splits(path) -> None:
-    """Writes the splits in use to a JSON file (tuning results for the next run)."""
+    """Writes the splits that are set to a JSON file (tuning results for the next run);
+    0 for the lengths that run their defaults."""
     import json
 
-    data = {str(t): get_split(t) for t in range(14, 24) if split_range(t)}
+    data = {str(t): int(library().ntt_split_chosen(t)) for t in range(14, 24) if split_range(t)}
     with open(path, "w") as f:
         json.dump(data, f, indent=1)
 
 
 def load_splits(path) -> dict:
-    """Applies splits saved by save_splits; returns them."""
+    """Applies splits saved by save_splits; returns {log_t: log_r} as get_split then has it."""
     import json
 
     with open(path) as f:
         data = {int(k): int(v) for k, v in json.load(f).items()}
     for t, r in data.items():
         set_split(t, r)
-    return data
+    return {t: get_split(t) for t in data}
 
 
 def _host(arr: np.ndarray, name: str) -> np.ndarray:

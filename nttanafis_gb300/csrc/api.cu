@@ -481,7 +481,9 @@ int ntt_timing_stop(float* ms, int capacity) {
 int ntt_split_set(int log_t, int log_r) {
     int lo = 0, hi = 0;
     if (!split_range(log_t, lo, hi) || (log_r != 0 && (log_r < lo || log_r > hi))) return -1;
-    const int prev = g_split[log_t].exchange(log_r);
+    // what ntt_split_get reports for the default restores it: a lone product's default is
+    // another split at some lengths, which a stored value would displace
+    const int prev = g_split[log_t].exchange(log_r == default_split(log_t) ? 0 : log_r);
     return prev ? prev : default_split(log_t);
 }
 
@@ -492,6 +494,16 @@ int ntt_split_get(int log_t) {
     if (!split_range(log_t, lo, hi)) return 0;
     const int o = g_split[log_t].load();
     return o ? o : default_split(log_t);
+}
+
+int ntt_split_chosen(int log_t) {
+    int lo = 0, hi = 0;
+    return split_range(log_t, lo, hi) ? g_split[log_t].load() : 0;
+}
+
+int ntt_split_lone(int log_t) {
+    int lo = 0, hi = 0;
+    return split_range(log_t, lo, hi) ? lone_log_r(log_t) : 0;
 }
 
 int ntt_split_range(int log_t, int* lo, int* hi) {
@@ -529,7 +541,8 @@ uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream) {
         const int before = g_split[log_t].load();
         float best = 1e30f, standard = 1e30f;
         int pick = 0;
-        for (int r = lo - 1; ok && r <= hi; ++r) {  // the default first, then every split
+        for (int r = lo - 1; ok && r <= hi; ++r) {  // the default first, then every other split
+            if (r == default_split(log_t)) continue;
             g_split[log_t].store(r < lo ? 0 : r);
             ok = ntt_mul_workspace_mul_device(ws, dst, na + nb, a, na, b, nb, st) == 1;  // tables, warm-up
             float ms = 1e30f;

@@ -108,6 +108,7 @@ int four_step_log_r(const Geom& g);
 // and 59.2, 1,048,576^2 138.5 and 142.9, its square 104.6 and 107.9, 700,001 x 650,003
 // 113.2 and 114.1; at 2^19 rows of 2^11 points gain for squares alone).
 int single_log_r(const Geom& g);
+int lone_log_r(int log_t);  // for a length on the lazy primes
 // Kernel constants of a plan with four-step split R = 2^log_r (tables built on
 // first use), or with the split in use.
 bool prepare_params(const Geom& g, int log_r, PrimeSet& ps, CrtParams& cp);

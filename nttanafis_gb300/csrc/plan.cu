@@ -454,11 +454,12 @@ static bool step_tables(int dev, u32 p, int log_t, int log_r, u32 cofactor, Step
 }
 
 // Four-step split of the lazy transforms: log2 R for each length 2^log_t, 0 for
-// the default (default_split). Set by ntt_split_set, e.g. from ntt_tune_splits.
+// the defaults (default_split, lone_log_r), never default_split's own value. Set by
+// ntt_split_set and ntt_tune_splits.
 std::atomic<int> g_split[kMaxLogT + 1];
 
 // Range of log2 R with column and row kernels for a lazy transform of 2^log_t
-// points (columns 2^7..2^11, rows 2^7..2^13); false when the length has no
+// points (columns 2^6..2^11, rows 2^7..2^13); false when the length has no
 // four-step form or is one of the wide lengths.
 bool split_range(int log_t, int& lo, int& hi) {
     if (log_t <= kMaxBlockLog || log_t > 23) return false;
@@ -475,12 +476,14 @@ int four_step_log_r(const Geom& g) {
     return o ? o : default_split(g.log_t);
 }
 
-int single_log_r(const Geom& g) {
-    if (g.log_t < kMaxBlockLog || g.log_t == 19 || g.wide || g.split()) return four_step_log_r(g);
-    const int o = g.log_t > kMaxBlockLog ? g_split[g.log_t].load(std::memory_order_relaxed) : 0;
+int lone_log_r(int log_t) {
+    if (log_t < kMaxBlockLog) return 0;
+    const int o = log_t > kMaxBlockLog ? g_split[log_t].load(std::memory_order_relaxed) : 0;
     if (o) return o;
-    return g.log_t <= 18 ? std::max(g.log_t - 10, 6) : std::min(g.log_t - 12, 10);
+    return log_t <= 19 ? std::max(log_t - 10, 6) : std::min(log_t - 12, 10);
 }
+
+int single_log_r(const Geom& g) { return g.wide || g.split() ? four_step_log_r(g) : lone_log_r(g.log_t); }
 
 // Fills the kernel constants of a plan whose four-step split is R = 2^log_r (0 for
 // the one-CTA lengths); builds missing tables on the current device.

@@ -188,3 +188,36 @@ def test_repeated_plans_are_identical_and_failures_repeat():
     c2 = ntt.ConvPlan.new(3000, 2000, 0xFFFF, 0xFFFF, False)
     assert c1 == c2 and c1 is not None
     assert ntt.ConvPlan.new(3000, 2000, 0xFFFF, 0xFFFF, True) != c1
+
+
+# log2 R of a lone product's default split, per log2 of the transform length
+LONE_DEFAULTS = {14: 6, 15: 6, 16: 6, 17: 7, 18: 8, 19: 9, 20: 8, 21: 9, 22: 10, 23: 10}
+
+
+def test_splits_set_back_and_loaded_restore_the_defaults(tmp_path):
+    lone = {t: ntt.lone_split(t) for t in LONE_DEFAULTS}
+    assert lone == LONE_DEFAULTS
+    assert ntt.lone_split(13) == 0 and ntt.lone_split(24) == 0
+    path = tmp_path / "splits.json"
+    for t in LONE_DEFAULTS:
+        lo, hi = ntt.split_range(t)
+        for r in range(lo, hi + 1):
+            previous = ntt.set_split(t, r)
+            assert ntt.get_split(t) == r
+            if r != previous:
+                assert ntt.lone_split(t) == r
+            ntt.set_split(t, previous)
+            assert ntt.get_split(t) == previous and ntt.lone_split(t) == LONE_DEFAULTS[t], (t, r)
+    ntt.save_splits(path)  # nothing is set
+    ntt.load_splits(path)
+    assert {t: ntt.lone_split(t) for t in LONE_DEFAULTS} == LONE_DEFAULTS
+    try:  # one length set, the others untouched
+        ntt.set_split(20, 11)
+        ntt.save_splits(path)
+        ntt.set_split(20, 0)
+        ntt.set_split(17, 9)
+        assert ntt.load_splits(path)[20] == 11
+        assert {t: ntt.lone_split(t) for t in LONE_DEFAULTS} == {**LONE_DEFAULTS, 20: 11}
+    finally:
+        ntt.set_split(20, 0)
+        ntt.set_split(17, 0)

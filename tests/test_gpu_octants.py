@@ -65,6 +65,20 @@ def test_octant_edges_in_every_lazy_column_kernel(gpu, ws, log_t, log_r):
             gpu.set_split(log_t, previous)
 
 
+# the splits that lone products run while none is set, and the 2^10-point columns of
+# lengths whose default is another
+@pytest.mark.parametrize("log_t,log_r", [(14, 6), (15, 6), (16, 6), (17, 7), (18, 8), (19, 9), (20, 8), (21, 9),
+                                         (18, 10), (19, 10)])
+def test_octant_edges_of_the_lone_defaults(gpu, ws, log_t, log_r):
+    if gpu.lone_split(log_t) != log_r:
+        gpu.set_split(log_t, log_r)
+    try:
+        assert gpu.lone_split(log_t) == log_r
+        test_octant_edges_in_every_lazy_column_kernel(gpu, ws, log_t, 0)
+    finally:
+        gpu.set_split(log_t, 0)
+
+
 @pytest.mark.parametrize("log_t,octants", [(22, 5), (22, 7), (23, 6), (24, 5), (24, 6), (24, 7), (25, 5)])
 def test_octants_of_the_wide_lengths(gpu, ws, log_t, octants):
     n = octants * (1 << log_t) // 8
