@@ -199,3 +199,23 @@ def test_inverse_at_every_group_size_with_zeros_among_the_elements(n, method):
         assert np.array_equal(one.cpu().numpy()[good], got[good])
     finally:
         field_module.mul_method(previous)
+
+
+@pytest.mark.parametrize("method", [0, 1])
+def test_powers_on_both_sides_of_the_window_rule(method):
+    # short exponents, sparse ones (square and multiply), ones whose windows save one
+    # product or many, the longest
+    from nttanafis_gb300 import field as field_module
+
+    previous = field_module.mul_method(method)
+    try:
+        f = next(ntt.PrimeField.catalog())
+        p = f.modulus
+        values = [0, 1, 2, p - 1, p - 2, 123456789012345, 1 << 49]
+        a, out = dev(values), empty(len(values))
+        for e in [0, 1, 7, 255, 256, 257, 319, 320, 322, 323, 1023, 1024, 3510, 65535, 65536, 65537, 1 << 40,
+                  (1 << 40) + 1, 2863311530, p - 2, p - 1, (1 << 63) + 5, (1 << 64) - 1]:
+            f.pow(out, a, e)
+            assert host(out) == [pow(v, e, p) for v in values], e
+    finally:
+        field_module.mul_method(previous)
