@@ -314,11 +314,13 @@ uint8_t ntt_crt_pair_combine_device(uint64_t first, uint64_t second, int64_t* d_
  * results.
  * ntt_tune_splits times every settable split of each length in [min_log_t, max_log_t] on
  * products that fill the transform on the lazy primes (balanced up to 2^21 points,
- * a 2^19-limb shorter operand above; `reps` products per timing, best of two) on
- * `stream` and keeps the fastest when it beats the default by 2%; it
- * synchronizes `stream` and allocates its operands for the call. Calls made by other
- * threads meanwhile may run with a split under trial (their results stay exact). No
- * reference counterpart: the reference fixes its geometry in Geometry::select. */
+ * a 2^19-limb shorter operand above), alone and as members of a batch, and on squares
+ * (`reps` calls per timing, best of two; the defaults first and last) on `stream`. It
+ * keeps the fastest for lone products when it beats the default by 2% there and no other
+ * kind loses 1%; it synchronizes `stream` and allocates its operands for the call. Calls
+ * made by other threads meanwhile may run with a split under trial (their results stay
+ * exact). No reference counterpart: the reference fixes its geometry in
+ * Geometry::select. */
 /* Products of single calls (workspace and plan calls; batches keep the transforms)
  * with a_len * b_len <= max_products limb products and at most 1,024 result limbs
  * take the direct column-sum basecase: one thread-block cluster of 1 to 8 CTAs, no

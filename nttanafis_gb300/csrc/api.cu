@@ -523,55 +523,88 @@ uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream) {
     // The timed products fill the transform on the lazy primes, whose splits these
     // are: balanced up to 2^21 points; above, a shorter operand of 2^19 limbs (a
     // balanced product there takes the wide primes, whose split is fixed).
-    constexpr int kLazyShortLog = 19;
-    const u64 full = (u64)1 << max_log_t;
+    constexpr int kLazyShortLog = 19, kLazySquareLog = 21;
+    constexpr u64 kMaxMembers = 16;
+    const u64 full = (u64)1 << max_log_t, results = std::max(full, (u64)1 << 20);
     u64 *a = nullptr, *b = nullptr, *dst = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ntt_mul_workspace* ws = ntt_mul_workspace_new();
-    bool ok = ws && cuda_ok(cudaMalloc(&a, full * 8), "cudaMalloc") && cuda_ok(cudaMalloc(&b, full / 2 * 8), "cudaMalloc") &&
-              cuda_ok(cudaMalloc(&dst, full * 8), "cudaMalloc") &&
+    ntt_batch* batch = ntt_batch_new();
+    bool ok = ws && batch && cuda_ok(cudaMalloc(&a, full * 8), "cudaMalloc") &&
+              cuda_ok(cudaMalloc(&b, full / 2 * 8), "cudaMalloc") &&
+              cuda_ok(cudaMalloc(&dst, results * 8), "cudaMalloc") &&
               cuda_ok(cudaEventCreate(&e0), "cudaEventCreate") && cuda_ok(cudaEventCreate(&e1), "cudaEventCreate") &&
               cuda_ok(cudaMemsetAsync(a, 0xA5, full * 8, st), "cudaMemset") &&
               cuda_ok(cudaMemsetAsync(b, 0x3C, full / 2 * 8, st), "cudaMemset");
+    if (ok) {
+        ntt_batch_set_graphs(batch, 0);
+        ntt_batch_set_lanes(batch, 1);
+    }
+    // The shortest of two runs of `reps` calls, after one that builds the tables.
+    auto time = [&](auto&& call) {
+        float best = 1e30f;
+        ok = ok && call();
+        for (int round = 0; ok && round < 2; ++round) {
+            ok = cuda_ok(cudaEventRecord(e0, st), "cudaEventRecord");
+            for (int i = 0; ok && i < reps; ++i) ok = call();
+            float t = 0;
+            ok = ok && cuda_ok(cudaEventRecord(e1, st), "cudaEventRecord") &&
+                 cuda_ok(cudaEventSynchronize(e1), "cudaEventSynchronize") &&
+                 cuda_ok(cudaEventElapsedTime(&t, e0, e1), "cudaEventElapsedTime");
+            best = std::min(best, t / reps);
+        }
+        return best;
+    };
     for (int log_t = min_log_t; ok && log_t <= max_log_t; ++log_t) {
         int lo = 0, hi = 0;
         if (!split_range(log_t, lo, hi) || lo == hi) continue;
         const u64 nb = (u64)1 << std::min(log_t - 1, log_t <= 21 ? log_t - 1 : kLazyShortLog);
         const u64 na = ((u64)1 << log_t) - nb;  // na + nb - 1 coefficients fill 2^log_t points
+        // Every kind of call runs the split that is set, and the kinds disagree (2^18 points,
+        // R = 2^6 against 2^8: lone products 29 and 32 us, squares 33 and 23), so a split
+        // has to suit them all: lone products, squares, and the members of a batch.
+        std::vector<ntt_request> members(std::min(kMaxMembers, results >> log_t));
+        for (size_t i = 0; i < members.size(); ++i)
+            members[i] = ntt_request{dst + (i << log_t), na + nb, a, b, na, nb, 0, 0, 0, 0};
+        struct Times {
+            float mul, sqr, batch;
+        };
+        auto measure = [&](int log_r) {
+            g_split[log_t].store(log_r);
+            Times t;
+            t.mul = time([&] { return ntt_mul_workspace_mul_device(ws, dst, na + nb, a, na, b, nb, st) == 1; });
+            t.sqr = log_t > kLazySquareLog ? 0.0f : time([&] {
+                return ntt_mul_workspace_sqr_device(ws, dst, na + nb, a, (u64)1 << (log_t - 1), st) == 1;
+            });
+            t.batch = time([&] { return ntt_batch_run_device(batch, members.data(), members.size(), st) == 1; });
+            return t;
+        };
         const int before = g_split[log_t].load();
-        float best = 1e30f, standard = 1e30f;
-        int pick = 0;
-        for (int r = lo - 1; ok && r <= hi; ++r) {  // the default first, then every other split
-            if (r == default_split(log_t)) continue;
-            g_split[log_t].store(r < lo ? 0 : r);
-            ok = ntt_mul_workspace_mul_device(ws, dst, na + nb, a, na, b, nb, st) == 1;  // tables, warm-up
-            float ms = 1e30f;
-            for (int round = 0; ok && round < 2; ++round) {
-                ok = cuda_ok(cudaEventRecord(e0, st), "cudaEventRecord");
-                for (int i = 0; ok && i < reps; ++i)
-                    ok = ntt_mul_workspace_mul_device(ws, dst, na + nb, a, na, b, nb, st) == 1;
-                float t = 0;
-                ok = ok && cuda_ok(cudaEventRecord(e1, st), "cudaEventRecord") &&
-                     cuda_ok(cudaEventSynchronize(e1), "cudaEventSynchronize") &&
-                     cuda_ok(cudaEventElapsedTime(&t, e0, e1), "cudaEventElapsedTime");
-                ms = std::min(ms, t / reps);
-            }
-            if (r < lo) {
-                standard = ms;
-            } else if (ms < best) {
-                best = ms;
-                pick = r;
-            }
-        }
+        // the defaults first and last, every other split between
+        Times standard = measure(0);
+        std::vector<std::pair<int, Times>> tried;
+        for (int r = lo; ok && r <= hi; ++r)
+            if (r != default_split(log_t)) tried.emplace_back(r, measure(r));
+        const Times again = measure(0);
         if (!ok) {  // a failed trial leaves the split as it was
             g_split[log_t].store(before);
             break;
         }
-        // another split only when it is at least 2% faster than the default
-        g_split[log_t].store(best < 0.98f * standard ? pick : 0);
+        standard = Times{std::min(standard.mul, again.mul), std::min(standard.sqr, again.sqr),
+                         std::min(standard.batch, again.batch)};
+        // another split only when products gain at least 2% and nothing else loses 1%
+        float best = 0.98f * standard.mul;
+        int pick = 0;
+        for (const auto& [r, t] : tried)
+            if (t.mul < best && t.sqr <= 1.01f * standard.sqr && t.batch <= 1.01f * standard.batch) {
+                best = t.mul;
+                pick = r;
+            }
+        g_split[log_t].store(pick);
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
+    if (batch) ntt_batch_free(batch);
     if (ws) ntt_mul_workspace_free(ws);
     if (a) cudaFree(a);
     if (b) cudaFree(b);

@@ -497,3 +497,37 @@ def test_poisoned_scratch_and_any_shape_order(gpu):
         assert w.mul(dst, operand(la, 121), operand(lb, 122))
         assert np.array_equal(dst, expected[(la, lb)]), (la, lb)
     w.close()
+
+
+def test_tuned_splits_slow_no_kind_of_call(gpu):
+    # one split serves lone products, squares and batch members: a tuned one may not make
+    # squares slower (2^18 points, R = 2^6 against 2^8: 33 and 23 us; products 29 and 32)
+    import torch
+
+    n = 1 << 17
+    ws = gpu.GpuMulWorkspace()
+    stream = torch.cuda.Stream()
+    a, dst = (torch.full((k,), 77, dtype=torch.int64, device="cuda") for k in (n, 2 * n))
+    torch.cuda.synchronize()
+
+    def best():
+        times = []
+        for _ in range(8):
+            t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            assert ws.sqr_device(dst, a, stream)
+            t0.record(stream)
+            for _ in range(20):
+                ws.sqr_device(dst, a, stream)
+            t1.record(stream)
+            t1.synchronize()
+            times.append(t0.elapsed_time(t1))
+        return min(times)
+
+    try:
+        gpu.tune_splits(18, 18, reps=5, stream=stream)
+        tuned = best()
+        gpu.set_split(18, 0)
+        assert tuned <= 1.2 * best()
+    finally:
+        gpu.set_split(18, 0)
+        ws.close()
