@@ -37,6 +37,7 @@ import json
 import os
 import subprocess
 import sys
+import tempfile
 import time
 from pathlib import Path
 
@@ -94,12 +95,11 @@ class ClockSampler:
     def __init__(self, gpu_index: int):
         self.gpu = gpu_index
         self.proc = None
-        self.path = ROOT / "gpurun_out" / f"clocks_bench_{gpu_index}.csv"
+        self.samples = ""
 
     def __enter__(self):
         try:
-            self.path.parent.mkdir(exist_ok=True)
-            self.fh = open(self.path, "w")
+            self.fh = tempfile.TemporaryFile("w+")
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--id={self.gpu}", f"--query-gpu={self.QUERY}", "--format=csv,noheader,nounits",
                  "-lms", "100"], stdout=self.fh, stderr=subprocess.DEVNULL)
@@ -115,14 +115,16 @@ class ClockSampler:
                 self.proc.wait(timeout=5)
             except Exception:
                 self.proc.kill()
+            self.fh.seek(0)
+            self.samples = self.fh.read()
             self.fh.close()
 
     def summary(self) -> dict:
-        if self.proc is None or not self.path.exists():
+        if self.proc is None:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"]}
         sms, maxes, reasons = [], [], set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for line in self.path.read_text().splitlines():
+        for line in self.samples.splitlines():
             parts = [p.strip() for p in line.split(",")]
             if len(parts) < 9:
                 continue
@@ -219,7 +221,8 @@ def run_reference(args) -> None:
     print(json.dumps(line), flush=True)
 
 
-KERNEL_NAMES = ["pack+column DIF (k_fwd_cols)", "row DIF+pointwise+DIT (k_rows)", "column DIT (k_inv_cols)",
+KERNEL_NAMES = ["pack+forward columns (k_fwd_cols)", "forward rows+pointwise+inverse rows (k_rows)",
+                "inverse columns (k_inv_cols)",
                 "CRT+window sums+look-back carry (k_crt_mul)"]
 
 
@@ -533,7 +536,8 @@ def run_gpu(args) -> None:
     splits = {}
     if not args.no_tune:
         try:
-            splits = ntt.tune_splits(14, 23, reps=3, stream=torch.cuda.current_stream(dev))
+            ntt.tune_splits(14, 23, reps=3, stream=torch.cuda.current_stream(dev))
+            splits = {t: ntt.lone_split(t) for t in range(14, 24)}
         except RuntimeError as exc:  # e.g. no room for the tuning operands: default splits
             print(f"split tuning skipped: {exc}", file=sys.stderr)
 
