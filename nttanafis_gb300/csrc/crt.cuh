@@ -28,10 +28,12 @@ __device__ __forceinline__ void crt_value(const u32 (&y)[NP], const CrtParams& c
     for (int i = 0; i < NP; ++i)
 #pragma unroll
         for (int d = 0; d < DM; ++d) col[d] += (u64)y[i] * cp.M[i][d];
-    // S/P to within 2^-16, from the high word of the top column of lazy primes (its
-    // digits are full there) or from the residues; X/P lies 1/4 from either end
+    // S/P to within 2^-16: from the high word of the top column of lazy primes, which with
+    // the columns below it leaves out at most 2^-20 of P for the sets that the planner
+    // takes (2^-16 for the eight smallest primes of the catalog), or from the residues.
+    // X/P lies 1/4 from either end.
     float f;
-        if constexpr (!WIDE && NP > 1) {
+    if constexpr (!WIDE && NP > 1) {
         f = (float)(u32)(col[DM - 1] >> 32) * cp.top;
     } else {
         f = 0.0f;

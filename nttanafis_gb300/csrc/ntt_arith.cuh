@@ -45,7 +45,9 @@ __device__ __forceinline__ u32 shoup_mul_add(u32 a, u32 x, u32 w, u32 wp, Mod m)
 // Returns x - m when x >= m, else x; valid when x < 2m and 2m <= 2^32.
 __device__ __forceinline__ u32 sub_if_ge(u32 x, u32 m) { return min(x, x - m); }
 
-// Montgomery product a*b*2^-32 mod p for a*b < 2^62 and p < 2^31; result in [0, 2p).
+// Montgomery product a*b*2^-32 mod p for a*b + 2^32 p < 2^64, below a*b / 2^32 + p: below
+// 3p for a < 4p, b < 2p of a lazy prime, below 2p for a < 2p, b < p of a wide one (the
+// largest, 2^31 - 2^24 + 1, leaves 1% of 2^64).
 __device__ __forceinline__ u32 mont_mul(u32 a, u32 b, u32 p, u32 pneg_inv) {
     const u64 t = (u64)a * b;
     const u32 m = (u32)t * pneg_inv;

@@ -289,13 +289,13 @@ __device__ __forceinline__ void dit_levels_cut(u32 (&x)[1][1 << RB], const uint2
     }
 }
 
-// One pass of RB forward levels starting at LEVEL over NV vectors of 2^LOG_N points,
-// VS words apart. Register block gg of a vector starts at block_start(gg) and spans
-// 2^RB points HQ apart. The first pass takes its twiddles from `first` (entries 1.. of
-// the shared roots), later ones from the pass table tw.
+// One pass of RB forward levels starting at LEVEL > 0 over NV vectors of 2^LOG_N points,
+// VS words apart (a first pass reads global memory, in the kernels). Register block gg of
+// a vector starts at block_start(gg) and spans 2^RB points HQ apart; tw is the pass table.
 template <class A, int LOG_N, int LEVEL, int RB, int NT, int NV, int VS, bool CUT = false>
-__device__ __forceinline__ void fwd_pass(u32* __restrict__ s, const uint2* __restrict__ tw,
-                                         const uint2* __restrict__ first, Mod m, int octs = kOctants) {
+__device__ __forceinline__ void fwd_pass(u32* __restrict__ s, const uint2* __restrict__ tw, Mod m,
+                                         int octs = kOctants) {
+    static_assert(LEVEL > 0, "the first pass has twiddles of its own");
     constexpr int E = 1 << RB;
     constexpr int LOG_HQ = LOG_N - LEVEL - RB;
     constexpr int HQ = 1 << LOG_HQ;
@@ -315,8 +315,7 @@ __device__ __forceinline__ void fwd_pass(u32* __restrict__ s, const uint2* __res
         for (int q = 0; q < VP; ++q)
 #pragma unroll
             for (int k = 0; k < E; ++k) x[q][k] = base[q * VS + slot_offset<HQ>(k)];
-        if constexpr (LEVEL == 0) fwd_levels<A, RB, 1, VP, true>(x, first, m);
-        else fwd_levels<A, RB, (1 << LEVEL), VP>(x, tw + (1 << LEVEL) + (i0 >> (LOG_HQ + RB)), m);
+        fwd_levels<A, RB, (1 << LEVEL), VP>(x, tw + (1 << LEVEL) + (i0 >> (LOG_HQ + RB)), m);
 #pragma unroll
         for (int q = 0; q < VP; ++q)
 #pragma unroll
@@ -362,16 +361,16 @@ __device__ __forceinline__ void dit_pass(u32* __restrict__ s, const uint2* __res
 #endif
 constexpr int kMaxRB = NTT_MAX_RB;
 
-// Full forward transform of NV vectors of 2^LOG_N points, VS words apart (from LEVEL
-// on); ends with a barrier.
-template <class A, int LOG_N, int NT, int NV, int VS, int LEVEL = 0, bool CUT = false>
-__device__ __forceinline__ void fwd_full(u32* s, const uint2* tw, const uint2* first, Mod m, int octs = kOctants) {
-    static_assert(!CUT || LEVEL >= 3, "a first pass in shared memory has no unused outputs");
+// The forward passes of NV vectors of 2^LOG_N points, VS words apart, from LEVEL > 0 on,
+// each followed by a barrier.
+template <class A, int LOG_N, int NT, int NV, int VS, int LEVEL, bool CUT = false>
+__device__ __forceinline__ void fwd_rest(u32* s, const uint2* tw, Mod m, int octs = kOctants) {
+    static_assert(!CUT || LEVEL >= 3, "an octant's points lie in whole register blocks");
     if constexpr (LEVEL < LOG_N) {
         constexpr int RB = LOG_N - LEVEL >= kMaxRB ? kMaxRB : LOG_N - LEVEL;
-        fwd_pass<A, LOG_N, LEVEL, RB, NT, NV, VS, CUT>(s, tw, first, m, octs);
+        fwd_pass<A, LOG_N, LEVEL, RB, NT, NV, VS, CUT>(s, tw, m, octs);
         __syncthreads();
-        fwd_full<A, LOG_N, NT, NV, VS, LEVEL + RB, CUT>(s, tw, first, m, octs);
+        fwd_rest<A, LOG_N, NT, NV, VS, LEVEL + RB, CUT>(s, tw, m, octs);
     }
 }
 
@@ -380,7 +379,7 @@ __device__ __forceinline__ void fwd_full(u32* s, const uint2* tw, const uint2* f
 template <class A, int LOG_N, int NT, int NV, int VS, int LEVEL, int END>
 __device__ __forceinline__ void fwd_range(u32* s, const uint2* tw, Mod m) {
     if constexpr (LEVEL < END) {
-        fwd_pass<A, LOG_N, LEVEL, kMaxRB, NT, NV, VS>(s, tw, nullptr, m);
+        fwd_pass<A, LOG_N, LEVEL, kMaxRB, NT, NV, VS>(s, tw, m);
         __syncthreads();
         fwd_range<A, LOG_N, NT, NV, VS, LEVEL + kMaxRB, END>(s, tw, m);
     }
@@ -394,22 +393,5 @@ __device__ __forceinline__ void dit_range(u32* s, const uint2* tw, Mod m, int oc
         dit_pass<A, LOG_N, LEVEL, kMaxRB, NT, NV, VS, CUT>(s, tw, m, octs);
         __syncthreads();
         dit_range<A, LOG_N, NT, NV, VS, LEVEL + kMaxRB, END, CUT>(s, tw, m, octs);
-    }
-}
-
-// Full inverse transform (unscaled); the short pass runs first. Ends with a barrier.
-template <class A, int LOG_N, int NT, int NV, int VS, int LEVEL = -1>
-__device__ __forceinline__ void dit_full(u32* s, const uint2* tw, Mod m) {
-    if constexpr (LEVEL < 0) {
-        constexpr int R0 = LOG_N % kMaxRB;
-        if constexpr (R0 > 0) {
-            dit_pass<A, LOG_N, 0, R0, NT, NV, VS>(s, tw, m);
-            __syncthreads();
-        }
-        dit_full<A, LOG_N, NT, NV, VS, R0>(s, tw, m);
-    } else if constexpr (LEVEL < LOG_N) {
-        dit_pass<A, LOG_N, LEVEL, kMaxRB, NT, NV, VS>(s, tw, m);
-        __syncthreads();
-        dit_full<A, LOG_N, NT, NV, VS, LEVEL + kMaxRB>(s, tw, m);
     }
 }

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kThreads) k_fwd_cols(const __grid_constant__ T
     }
     if (CHECK && bad) votes[(blockIdx.x + threadIdx.x) % kAdmitSlots] = 1u;
     __syncthreads();
-    fwd_full<A, LOG_R, kThreads, M::G, M::VS, kMaxRB, CUT>(sm, tw, nullptr, pp.mod, octs);
+    fwd_rest<A, LOG_R, kThreads, M::G, M::VS, kMaxRB, CUT>(sm, tw, pp.mod, octs);
     // Four-step twiddle w_T^(col * brev(row)) = fa * fb[col][brev(k)], then the store.
     u32* dst = m.spec + ((size_t)(op * g.np + prime) << g.log_t) + first;
     const uint2* fbc = fb + M::col() * (M::SWEEPS + 1);
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(kCol4Threads, kCol4LogG == 2 ? 2 : 1)
         u32 x[1][E];
 #pragma unroll
         for (int k = 0; k < E; ++k) x[0][k] = __ldcg(q + ((u64)k << log_c));
-        dit_levels<A, 6, 1, 1, 2>(x, tw, pp.mod);  // the row pass wrote [0, 2p) ([0, p) when wide)
+        dit_levels<A, 6, 1, 1, 2>(x, tw, pp.mod);  // the row pass wrote [0, 2p)
         u32* base = sm + c * VS + 65 * blk;
 #pragma unroll
         for (int k = 0; k < E; ++k) base[k] = x[0][k];
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(kCol4Threads, 1) k_inv_cols4p(const __grid_con
             const u32* raw = sm + RB * blk + c;
 #pragma unroll
             for (int k = 0; k < E; ++k) x[0][k] = raw[8 * k];
-            dit_levels<A, 6, 1, 1, 2>(x, tw + 64 * prime, pp.mod);  // [0, 2p) in ([0, p) when wide)
+            dit_levels<A, 6, 1, 1, 2>(x, tw + 64 * prime, pp.mod);  // [0, 2p) in
         }
         __syncthreads();  // every raw read is done before the padded layout overwrites it
         if (used) {
