@@ -124,3 +124,52 @@ def test_dependent_block_splits_on_one_stream(gpu):
         for dsts in outs:
             assert torch.equal(dsts[k], want), SPLITS[k]
     ws.close()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("la,lb", [(40, 40), (1000, 731), (4000, 4000), (20000, 6007), (300000, 200000), (1 << 20, 1000)])
+def test_an_operand_that_arrives_by_an_event(gpu, la, lb, captured):
+    # the product's first kernel is launched dependently on the product before it in its
+    # stream, and must still wait for the other stream's event
+    import torch
+
+    ws = gpu.GpuMulWorkspace()
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+    x, y = operand(la, 3), operand(lb, 4)
+    src, b = (torch.from_numpy(v.view(np.int64)).cuda() for v in (x, y))
+    a = torch.zeros_like(src)
+    before, dst = (torch.empty(n, dtype=torch.int64, device="cuda") for n in (la + 2 * lb, la + lb))
+
+    def work():
+        assert ws.mul_device(before, a, b, main), gpu.last_error()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(400_000)  # a fifth of a millisecond
+            a.copy_(src)
+        assert ws.mul_device(before, b, b, main), gpu.last_error()
+        main.wait_stream(side)
+        assert ws.mul_device(dst, a, b, main), gpu.last_error()
+        with torch.cuda.stream(main):
+            a.zero_()
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(main):
+        work()
+    main.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=main):
+            work()
+    want = torch.from_numpy(oracle.mul(x, y, 4).view(np.int64)).cuda()
+    for _ in range(5):
+        dst.fill_(-1)
+        torch.cuda.synchronize()
+        if captured:
+            graph.replay()
+        else:
+            work()
+        torch.cuda.synchronize()
+        assert torch.equal(dst, want)
+    if captured:
+        del graph
+    ws.close()
