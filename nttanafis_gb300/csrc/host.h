@@ -103,8 +103,9 @@ int four_step_log_r(const Geom& g);
 // is four-step with 2^6-point columns too, where one CTA per prime would leave all but
 // five SMs idle; batch members of that length keep the one-CTA kernels.
 // From 2^20 points on it has rows of 2^12 points, so that the columns stay short: those
-// of 2^8 and 2^9 points take 40 registers a thread in their two passes, those of 2^10
-// points 64 (against 2^10-point columns: 524,288^2 72.6 and 76.8 us, 524,288 squared 56.4
+// of 2^8 points take 40 registers a thread in their two passes, those of 2^9 points run
+// CTAs of 128 threads, half as many as those of 2^10 points, at the same 64 registers
+// (against 2^10-point columns: 524,288^2 72.6 and 76.8 us, 524,288 squared 56.4
 // and 59.2, 1,048,576^2 138.5 and 142.9, its square 104.6 and 107.9, 700,001 x 650,003
 // 113.2 and 114.1; at 2^19 rows of 2^11 points gain for squares alone).
 int single_log_r(const Geom& g);

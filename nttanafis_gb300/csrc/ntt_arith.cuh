@@ -26,7 +26,7 @@ typedef uint64_t u64;
 // A modulus p and its negative n = 2^32 - p. Both come from memory, so that a
 // product is subtracted as a multiply-add by n: written as `- q * p`, the compiler
 // multiplies, then subtracts, one instruction more on the path that bounds the
-// transforms (register-only butterflies per clock and SM: 10.2 against 11.5 forward).
+// transforms (10.2 against 11.5 register-only Gentleman-Sande butterflies per clock and SM).
 struct Mod {
     u32 p, n;
 };
@@ -61,7 +61,8 @@ struct LazyArith {
     // x, y in [0, 4p) -> x + y*w, x - y*w in [0, 4p). With a = x below 2p, x' = a + y*w
     // keeps the multiply-adds whole and y' = 2a + 2p - x' is one three-input addition
     // more: 13.3 register-only butterflies per clock and SM, against 10.0 with y*w
-    // formed first and 11.5 for the Gentleman-Sande form ((x - y) * w).
+    // formed first and 11.5 for the Gentleman-Sande form ((x - y) * w), with twiddles per
+    // thread; probe.cu, whose twiddles are the same in every thread, runs this form at 14.3.
     static __device__ __forceinline__ void bf(u32& x, u32& y, uint2 w, Mod m) {
         const u32 a = sub_if_ge(x, m.p << 1);
         x = shoup_mul_add(a, y, w.x, w.y, m);
@@ -105,7 +106,8 @@ struct WideArith {
     static constexpr bool kWide = true;
     static __device__ __forceinline__ u32 red(u32 x, Mod m) { return min(x, x + m.n); }
     // x, y in [0, 2p) -> x + y*w, x - y*w in [0, 2p): both terms reduced to [0, p), the
-    // sums left open (2p < 2^32).
+    // sums left open (2p < 2^32). 13.4 register-only butterflies per clock and SM in the
+    // probe that runs the lazy ones at 14.3.
     static __device__ __forceinline__ void bf(u32& x, u32& y, uint2 w, Mod m) {
         const u32 a = red(x, m);
         const u32 t = red(shoup_mul(y, w.x, w.y, m), m);

@@ -184,9 +184,14 @@ constexpr u64 kMaxSplitLimbs = (u64)1 << 40;
 // addition and about ten more launches and copies, against 3 * 2^K * K for one
 // transform of the whole product. Returns the chosen k, or 0 when one transform is
 // within the margin. Measured on GB300 (per call, split against one transform):
-// 1,048,576 x 1,024 99 against 160 us, 4,194,304 x 524,288 477 against 797 us,
-// 1,048,576 x 131,072 149 against 165 us; below, the fixed part dominates
-// (20,000 x 300: 41 against 24 us; 16,384 x 4,096: 51 against 24 us).
+// 1,048,576 x 1,024 70 against 98 us, 4,194,304 x 32,768 270 and 421, 4,194,304 x 524,288
+// 398 and 428, 2,097,152 x 131,072 177 and 196; not split, for the fixed part or the second
+// transform per block: 16,384 x 4,096 33 against 20 us, 131,072 x 512 28 and 23,
+// 262,144 x 16,384 44 and 35, 1,500,000 x 150,000 142 and 129. The constants were fitted
+// before products left out the octants that they do not need: where the whole product
+// fills little more than half of its transform the rule still prices all of it, and splits
+// some that one transform would serve better (600,000 x 50,000 65 against 57 us,
+// 524,288 x 32,768 58 and 54, 1,048,576 x 131,072 103 and 100).
 #ifndef NTT_SPLIT_MARGIN
 #define NTT_SPLIT_MARGIN 0.8
 #endif

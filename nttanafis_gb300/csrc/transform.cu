@@ -801,7 +801,7 @@ __global__ void __launch_bounds__(row_threads(LOG_C)) k_rows(const __grid_consta
     }
 }
 
-// Column pass of the inverse four-step: column DIT, canonical residues in place.
+// Column pass of the inverse four-step: inverse columns, canonical residues in place.
 template <class A, int LOG_R, bool CUT>
 __global__ void __launch_bounds__(kThreads) k_inv_cols(const __grid_constant__ TransformArgs g) {
     extern __shared__ u32 sm[];
@@ -957,8 +957,8 @@ static size_t col2_smem(bool fwd) {
     return (size_t)K::G * K::VS * sizeof(u32) + (fwd ? (K::G * (K::EB + 1) + roots) * sizeof(uint2) : 0);
 }
 
-// One preference for the passes of lengths up to 2^19, the driver's for longer ones
-// (transform_common.cuh).
+// One preference for the columns and rows that lengths up to 2^19 run, the driver's for
+// longer ones (transform_common.cuh, kCarveout).
 static constexpr int col_carveout(int log_r) { return log_r <= 9 ? kCarveout : -1; }
 static constexpr int row_carveout(int log_c) { return log_c <= 10 ? kCarveout : -1; }
 

@@ -13,15 +13,18 @@ constexpr int kThreads = kColThreads;
 // hold on sm_103a).
 constexpr int kSmemOptIn = 200 * 1024;
 
-// Preferred shared-memory carveout of the one-CTA kernels and of the column and row
-// passes that the lengths up to 2^19 use (percent of the 228 KB an SM can give:
+// Preferred shared-memory carveout of the one-CTA kernels, of columns up to 2^9 points
+// and of rows up to 2^10, which are the passes of the lengths up to 2^19 (percent of the 228 KB an SM can give:
 // 132 KB). An SM drains before its split between L1 and shared memory changes, so
 // kernels with different preferences cannot overlap: with the driver's choice per
 // kernel, programmatic dependent launch stalled for whole kernels (65,536^2 32.9 us,
 // 23.5 with one preference; 260,000^2 57.5, 51.4; 164 KB there 55.5). Longer
-// transforms spend their time inside the kernels and keep the driver's choice, which
-// suits each one (4M^2: 671 us; 672 with 132 KB everywhere, 733 with 196 KB, whose L1
-// no longer holds the twiddles).
+// transforms spend their time inside the kernels and their rows keep the driver's choice,
+// which suits each one (4M^2: 671 us; 672 with 132 KB everywhere, 733 with 196 KB, whose
+// L1 no longer holds the twiddles). Lone products of 2^20 and 2^21 points run 2^8- and
+// 2^9-point columns with the preference between 2^12-point rows without it; that costs
+// nothing there (1,048,576^2 139.2 us so, with the driver's choice for both, and with the
+// preference for both; its square 103.6 each way, 524,288^2 72.2, 72.1 and 72.2).
 constexpr int kCarveout = 58;
 
 template <class A, bool SIGNED>
