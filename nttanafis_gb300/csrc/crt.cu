@@ -112,13 +112,12 @@ __global__ void __launch_bounds__(kCrtThreads, WIDE ? 6 : 5) k_crt_mul(const u32
                                                           u64 conv_len, u64 out_len, u64* __restrict__ dst,
                                                           u32* __restrict__ flags,
                                                           const __grid_constant__ CrtParams cp,
-                                                          const ProductDesc* batch,
+                                                          const ProductDesc* batch, bool chained,
                                                           u32* __restrict__ status) {
     constexpr int L = crt_limb_words(NP);
-    // the residues and cleared flags of the transform before it, and in a block split the
-    // descriptors (no __restrict__: they are not constant while the kernel waits)
-    wait_prior_grid();
-    release_dependents();  // the next product's first kernel
+    // a block split's descriptors, which a kernel of the sequence writes (no __restrict__:
+    // they are not constant while this one waits)
+    if (chained) wait_prior_grid();
     if (batch) {  // member blockIdx.y of a batch: grid.x covers its largest member
         const ProductDesc& d = batch[blockIdx.y];
         resid = d.spec;
@@ -127,6 +126,8 @@ __global__ void __launch_bounds__(kCrtThreads, WIDE ? 6 : 5) k_crt_mul(const u32
         dst = d.dst;
         flags = reinterpret_cast<u32*>(d.agg);
     }
+    wait_prior_grid();  // the residues and cleared flags of the transform before it
+    release_dependents();  // the next product's first kernel
     // Tiles are numbered in the order CTAs start, so a tile only ever waits for
     // tiles whose CTAs are already running.
     __shared__ u32 s_tile;
@@ -383,17 +384,17 @@ static cudaError_t crt_mul_any(const CrtParams& cp, dim3 grid, cudaStream_t st, 
     }
 }
 
-cudaError_t launch_crt_mul_batch(const ProductDesc* batch, int count, int max_tiles, int log_t,
+cudaError_t launch_crt_mul_batch(const ProductDesc* batch, int count, bool chained, int max_tiles, int log_t,
                                  const CrtParams& cp, cudaStream_t st, u32* status) {
     return crt_mul_any(cp, dim3(max_tiles, count), st, (const u32*)nullptr, log_t, (u64)0, (u64)0,
-                       (u64*)nullptr, (u32*)nullptr, cp, batch, status);
+                       (u64*)nullptr, (u32*)nullptr, cp, batch, chained, status);
 }
 
 cudaError_t launch_crt_mul(const u32* resid, int log_t, u64 conv_len, u64 out_len, u64* dst, uint8_t* agg,
                            const CrtParams& cp, cudaStream_t st, void (*mark)(cudaStream_t), u32* status) {
     const int tiles = (int)((out_len + kCrtTile - 1) / kCrtTile);
     const cudaError_t e = crt_mul_any(cp, dim3(tiles), st, resid, log_t, conv_len, out_len, dst,
-                                      reinterpret_cast<u32*>(agg), cp, (const ProductDesc*)nullptr, status);
+                                      reinterpret_cast<u32*>(agg), cp, (const ProductDesc*)nullptr, false, status);
     if (mark) mark(st);
     return e;
 }

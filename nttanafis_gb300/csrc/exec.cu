@@ -16,7 +16,7 @@ namespace ntt {
 // primes, sign and square) whose descriptors sit in device memory; max_len is the
 // longest member output (limbs of a product, coefficients of a convolution).
 bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 max_len, cudaStream_t st,
-                 u32* status, u32* shared_spec, const u64* shared, u64 shared_len) {
+                 u32* status, const SplitBlocks* split) {
     TransformArgs ta;
     memset(&ta, 0, offsetof(TransformArgs, ps));
     CrtParams cp;
@@ -24,9 +24,14 @@ bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 m
     if (!prepare_params(g0, log_r, ta.ps, cp)) return false;
     ta.batch = descs;
     ta.count = n;
-    ta.shared_spec = shared_spec;
-    ta.a_only = shared_spec ? 1 : 0;
-    ta.cut = shared_spec ? 0 : 1;  // a block product fills its transform
+    ta.cut = 1;
+    if (split) {
+        ta.shared_spec = split->spectrum;
+        ta.arena = split->arena;
+        ta.arena_step = split->step;
+        ta.a_only = 1;
+        ta.cut = 0;  // a block product fills its transform
+    }
     ta.np = g0.np;
     ta.log_t = g0.log_t;
     ta.wide = g0.wide;
@@ -41,7 +46,7 @@ bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 m
         if (!cuda_ok(launch_clear_votes_batch(descs, n, st), "batched vote clearing launch")) return false;
         mark(st);
     }
-    if (!shared_spec && !g0.conv && g0.log_t <= kFusedMaxLog && g0.np == kFusedPrimes && !g0.wide) {
+    if (!split && !g0.conv && g0.log_t <= kFusedMaxLog && g0.np == kFusedPrimes && !g0.wide) {
         note_launches(1);
         const bool ok = cuda_ok(launch_small_fused(ta, cp, sq, st), "batched fused product launch");
         mark(st);
@@ -49,7 +54,7 @@ bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 m
     }
     if (g0.log_t <= kMaxBlockLog) {
         note_launches(1);
-        if (!cuda_ok(launch_small(ta, shared_spec ? kRowPre : sq ? kRowSqr : kRowMul, sign, st),
+        if (!cuda_ok(launch_small(ta, split ? kRowPre : sq ? kRowSqr : kRowMul, sign, st),
                      "batched transform launch"))
             return false;
         mark(st);
@@ -57,11 +62,12 @@ bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 m
         ta.log_r = log_r;
         ta.log_c = g0.log_t - ta.log_r;
         note_launches(3);
+        const bool shared = split && split->shared;
         if (shared) {  // the shared factor's columns with the members', then its rows
             ta.with_args = 1;
-            ta.a = ta.b = shared;
-            ta.la = ta.lb = shared_len;
-            ta.spec = shared_spec;
+            ta.a = ta.b = split->shared;
+            ta.la = ta.lb = split->shared_len;
+            ta.spec = split->spectrum;
         }
         if (!cuda_ok(launch_fwd_cols(ta, sq, sign, st), "batched column pass launch")) return false;
         mark(st);
@@ -72,7 +78,7 @@ bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 m
             mark(st);
             ta.batch = descs;
         }
-        if (!cuda_ok(launch_rows(ta, shared_spec ? kRowPre : sq ? kRowSqr : kRowMul, st), "batched row pass launch"))
+        if (!cuda_ok(launch_rows(ta, split ? kRowPre : sq ? kRowSqr : kRowMul, st), "batched row pass launch"))
             return false;
         mark(st);
         if (!cuda_ok(launch_inv_cols(ta, st), "batched inverse column pass launch")) return false;
@@ -81,8 +87,8 @@ bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 m
     note_launches(1);
     const bool ok =
         g0.conv ? cuda_ok(launch_crt_conv_batch(descs, n, max_len, g0.log_t, cp, st, status), "batched CRT launch")
-                : cuda_ok(launch_crt_mul_batch(descs, n, (int)((max_len + kCrtTile - 1) / kCrtTile), g0.log_t, cp, st,
-                                               status),
+                : cuda_ok(launch_crt_mul_batch(descs, n, split != nullptr, (int)((max_len + kCrtTile - 1) / kCrtTile),
+                                               g0.log_t, cp, st, status),
                           "batched CRT launch");
     mark(st);
     return ok;
@@ -131,12 +137,12 @@ static bool execute_split(const Geom& g, const u64* d_a, const u64* d_b, u64* d_
     const u64 chunk = g.split_chunk();
     for (u64 first = 0; first < g.blocks; first += chunk) {
         const u64 count = std::min(chunk, g.blocks - first);
-        const bool shared = first == 0 && !one_cta;
+        const SplitBlocks split{spectrum, (u32*)arena, member / sizeof(u32), first == 0 && !one_cta ? sht : nullptr, S};
         note_launches(1);
         if (!cuda_ok(launch_split_descs(descs, first, count, lng, L, sht, S, g.block, d_dst, odd, arena, member, spec,
                                         flags, first == 0 ? carry_flag_words(g.out_len) : 0, st),
                      "split descriptors") ||
-            !run_members(descs, (int)count, g, false, g.block + S, st, status, spectrum, shared ? sht : nullptr, S))
+            !run_members(descs, (int)count, g, false, g.block + S, st, status, &split))
             return false;
     }
     note_launches(1);

@@ -125,12 +125,17 @@ bool kernels_ready();
 
 // The kernels of n batch members of one transform class, descriptors in device
 // memory; convolution members are admitted on the device (their votes).
-// status: the failure bytes of launch.h, or null. shared_spec: the stored spectrum
-// of a factor all members share (block-split products), or null. shared: that factor
-// itself (shared_len limbs), when its spectrum is still to be made, with the members'
-// (four-step lengths), or null.
+// status: the failure bytes of launch.h, or null. split: the members are blocks of a
+// split product, whose descriptors a kernel ahead on `st` writes.
+struct SplitBlocks {
+    u32* spectrum;      // of the shorter operand, which all blocks share
+    u32* arena;         // residues of the blocks, `step` words apart
+    u64 step;
+    const u64* shared;  // the shorter operand (shared_len limbs) when its spectrum is still
+    u64 shared_len;     // to be made, with the members' (four-step lengths), or null
+};
 bool run_members(const ProductDesc* descs, int n, const Geom& g0, bool sq, u64 max_len, cudaStream_t st,
-                 u32* status = nullptr, u32* shared_spec = nullptr, const u64* shared = nullptr, u64 shared_len = 0);
+                 u32* status = nullptr, const SplitBlocks* split = nullptr);
 // Products of single calls with at most this many limb products (a_len * b_len)
 // take the direct column-sum basecase (school.cu) when it holds them; 0 turns it
 // off. Set by ntt_school_set.

@@ -107,6 +107,10 @@ struct TransformArgs {
     // kRowPre; a_only: the members' column passes transform operand a alone.
     u32* shared_spec;
     int a_only;
+    // Residues of a block split's members: member i's at arena + i * arena_step (words), or
+    // null (a batch: the descriptors').
+    u32* arena;
+    u64 arena_step;
     // 1: the members' column pass transforms one more operand, the one that the fields
     // a, la and spec describe (the shorter operand, with the first blocks).
     int with_args;
@@ -216,8 +220,9 @@ cudaError_t launch_crt_conv(const u32* resid, int log_t, u64 conv_len, u64* dst,
                             u32* status = nullptr);
 // Batched forms: every member of `batch` (device array of `count` descriptors)
 // shares log_t and the prime set of `cp`. Convolution members with votes are
-// written only when admitted.
-cudaError_t launch_crt_mul_batch(const ProductDesc* batch, int count, int max_tiles, int log_t,
+// written only when admitted. chained: the descriptors come from a kernel of the same
+// sequence (a block split's) and are read after the kernel's wait.
+cudaError_t launch_crt_mul_batch(const ProductDesc* batch, int count, bool chained, int max_tiles, int log_t,
                                  const CrtParams& cp, cudaStream_t st, u32* status = nullptr);
 cudaError_t launch_crt_conv_batch(const ProductDesc* batch, int count, u64 max_conv_len, int log_t,
                                   const CrtParams& cp, cudaStream_t st, u32* status = nullptr);
@@ -297,8 +302,9 @@ void set_last_error(const std::string& message);
 // launch then overlaps the end of whatever ran before it, the product before it above
 // all (whose last kernel releases it early). The first kernel of a batch class is not
 // (first_dependent): its descriptors are copied in ahead of it, so the row and inverse
-// column passes of the class read them before they wait. Those of a block split come from
-// a kernel of the sequence (k_split_descs), and every pass reads them after its wait.
+// column passes and the CRT of the class read them before they wait. Those of a block split
+// come from a kernel of the sequence (k_split_descs), and every pass that reads them waits
+// first (member_after, and `chained` of k_crt_mul).
 // Both device calls are no-ops for a kernel launched without the attribute.
 // What an earlier kernel wrote is read with __ldcg, not through the read-only path
 // (__ldg): it may be written while the kernel that reads it is already running.

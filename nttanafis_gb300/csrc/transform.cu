@@ -330,8 +330,7 @@ __global__ void __launch_bounds__(Columns<LOG_R>::NT, Columns<LOG_R>::MINB)
     const int prime = blockIdx.y;
     const PrimeParams& pp = g.ps.pr[prime];
     release_dependents();
-    if (g.shared_spec) wait_prior_grid();  // descriptors that a kernel of the sequence wrote
-    const Member m = member_of(g, blockIdx.z, false);
+    const Member m = member_after(g, blockIdx.z, false);
     const int octs = CUT ? octants_of(m.conv_len, g.log_t) : kOctants;
     const int log_c = g.log_c;
     const int c = threadIdx.x & (G - 1), blk = threadIdx.x >> K::LOG_G;
@@ -501,8 +500,7 @@ __global__ void __launch_bounds__(kCol4Threads, kCol4LogG == 2 ? 2 : 1)
     const int prime = blockIdx.y;
     const PrimeParams& pp = g.ps.pr[prime];
     release_dependents();
-    if (g.shared_spec) wait_prior_grid();  // descriptors that a kernel of the sequence wrote
-    const Member m = member_of(g, blockIdx.z, false);
+    const Member m = member_after(g, blockIdx.z, false);
     const int octs = CUT ? octants_of(m.conv_len, g.log_t) : kOctants;
     const int log_c = g.log_c;
     const int c = threadIdx.x & (G - 1), blk = threadIdx.x >> LOG_G;
@@ -683,15 +681,13 @@ __global__ void __launch_bounds__(row_threads(LOG_C)) k_rows(const __grid_consta
     const int prime = blockIdx.y;
     const int row0 = blockIdx.x << LOG_RPC;
     const PrimeParams& pp = g.ps.pr[prime];
-    // Blocks of a split product (kRowPre): descriptors that a kernel of the sequence wrote,
-    // read after the wait. Their transforms are filled (no cut).
-    Member m;
-    if constexpr (MODE != kRowPre) m = member_of(g, blockIdx.z, NV == 1);
+    const Member m = member_after(g, blockIdx.z, NV == 1);
     if constexpr (!kRowsReleaseLate<LOG_C>) release_dependents();
     // rows of octants that the member's coefficients do not need (a CTA whose first row
     // is needed may hold unneeded ones as well: what it makes of them is not read)
-    if constexpr (MODE != kRowPre)
-        if (g.cut && row0 >= octants_of(m.conv_len, g.log_t) << (g.log_r - 3)) return;
+    if (g.cut && row0 >= octants_of(m.conv_len, g.log_t) << (g.log_r - 3)) return;
+    u32* ra = m.spec + ((size_t)prime << g.log_t) + ((size_t)row0 << LOG_C);
+    const u32* rb = m.spec + ((size_t)(g.np + prime) << g.log_t) + ((size_t)row0 << LOG_C);
     // the stored spectrum of the rows (kRowFwd writes it, kRowPre multiplies by it)
     u32* rs = g.shared_spec + ((size_t)prime << g.log_t) + ((size_t)row0 << LOG_C);
     // The rows' inverse four-step factors: RPC x 64 low-digit entries, RPC x C/64 high.
@@ -705,9 +701,6 @@ __global__ void __launch_bounds__(row_threads(LOG_C)) k_rows(const __grid_consta
     }
     wait_prior_grid();  // the column pass's output
     if constexpr (kRowsReleaseLate<LOG_C>) release_dependents();
-    if constexpr (MODE == kRowPre) m = member_of(g, blockIdx.z, true);
-    u32* ra = m.spec + ((size_t)prime << g.log_t) + ((size_t)row0 << LOG_C);
-    const u32* rb = m.spec + ((size_t)(g.np + prime) << g.log_t) + ((size_t)row0 << LOG_C);
     // First forward pass: global -> shared. Block gg of a row holds points gg + k * HQ.
     {
         constexpr int LOG_HQ = LOG_C - RB;
@@ -811,8 +804,7 @@ __global__ void __launch_bounds__(kThreads) k_inv_cols(const __grid_constant__ T
     const int prime = blockIdx.y;
     const PrimeParams& pp = g.ps.pr[prime];
     release_dependents();
-    if (g.shared_spec) wait_prior_grid();  // descriptors that a kernel of the sequence wrote
-    const Member m = member_of(g, blockIdx.z, false);
+    const Member m = member_after(g, blockIdx.z, false);
     const int octs = CUT ? octants_of(m.conv_len, g.log_t) : kOctants;
     const u64 step = (u64)M::RS << g.log_c;
     u32* const base = m.spec + ((size_t)prime << g.log_t) + ((u64)M::row0() << g.log_c) +
@@ -1037,8 +1029,8 @@ static cudaError_t inv_cols_cut(const TransformArgs& g, cudaStream_t st, bool in
             return e == cudaSuccess ? opt_in(k, col_carveout(L)) : e;
         }
         // members of a batch start on 256-byte boundaries, blocks of a split product a
-        // multiple of 256 bytes after the shorter operand's spectrum in the caller's scratch
-        const u32* first = g.batch ? g.shared_spec : g.spec;
+        // multiple of 256 bytes apart in the caller's scratch
+        const u32* first = g.batch ? g.arena : g.spec;
         if ((reinterpret_cast<uintptr_t>(first) & 15) != 0)
             return launch_dependent(k, grid, dim3(kCol4Threads), col4_smem(false), st, g);
         const unsigned items = grid.x * grid.y * grid.z;

@@ -57,6 +57,16 @@ __device__ __forceinline__ Member member_of(const TransformArgs& g, int idx, boo
     return Member{g.a, g.b, g.la, g.lb, g.spec, g.conv_len, square};
 }
 
+// The member for the passes after the first, which may not have waited for every kernel of
+// the sequence yet. A batch's descriptors were copied in ahead of the first kernel; those
+// of a block split are written by one, but its residues are evenly spaced and its
+// transforms filled, so these passes need none.
+__device__ __forceinline__ Member member_after(const TransformArgs& g, int idx, bool square) {
+    if (g.batch && g.arena)
+        return Member{nullptr, nullptr, 0, 0, g.arena + idx * g.arena_step, (u64)1 << g.log_t, square};
+    return member_of(g, idx, square);
+}
+
 // Admission votes of a convolution (src/convolve.rs:169-184) checked by the forward
 // column passes as they load the coefficients: the votes and bound of operand op
 // of a member, or null when the CTA checks nothing. Only prime 0's CTAs check, as
