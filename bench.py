@@ -214,6 +214,7 @@ def run_reference(args) -> None:
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
         "data": "synthetic (SplitMix64 seeds 1, 2)",
         "config": {"workload": WORKLOAD, "la": LA, "lb": LB, "l2": "n/a (CPU)"},
+        "reference_kind": "port: a C restatement of the algorithm; the Rust crate cannot be built here",
         "cpu_baseline": {"value": value, "unit": "products/s", "cores": threads, "kind": "port",
                          "sample": f"{args.steps} whole 1M x 1M products, {threads} threads, {cpu_model()}"},
         "e2e": {"value": value, "unit": "products/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},

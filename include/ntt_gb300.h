@@ -315,7 +315,7 @@ uint8_t ntt_crt_pair_combine_device(uint64_t first, uint64_t second, int64_t* d_
  * ntt_tune_splits times every settable split of each length in [min_log_t, max_log_t] on
  * products that fill the transform on the lazy primes (balanced up to 2^21 points,
  * a 2^19-limb shorter operand above), alone and as members of a batch, and on squares
- * (`reps` calls per timing, best of two; the defaults first and last) on `stream`. It
+ * (`reps` calls per timing, best of five; the defaults first and last) on `stream`. It
  * keeps the fastest for lone products when it beats the default by 2% there and no other
  * kind loses 1%; it synchronizes `stream` and allocates its operands for the call. Calls
  * made by other threads meanwhile may run with a split under trial (their results stay

@@ -524,7 +524,7 @@ uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream) {
     // are: balanced up to 2^21 points; above, a shorter operand of 2^19 limbs (a
     // balanced product there takes the wide primes, whose split is fixed).
     constexpr int kLazyShortLog = 19, kLazySquareLog = 21;
-    constexpr u64 kMaxMembers = 16;
+    constexpr int kMaxMembers = 16;
     const u64 full = (u64)1 << max_log_t, results = std::max(full, (u64)1 << 20);
     u64 *a = nullptr, *b = nullptr, *dst = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -540,11 +540,12 @@ uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream) {
         ntt_batch_set_graphs(batch, 0);
         ntt_batch_set_lanes(batch, 1);
     }
-    // The shortest of two runs of `reps` calls, after one that builds the tables.
+    // The shortest of five runs of `reps` calls, after one that builds the tables: a run of
+    // a few short calls varies by some percent with what the host takes to start it.
     auto time = [&](auto&& call) {
         float best = 1e30f;
         ok = ok && call();
-        for (int round = 0; ok && round < 2; ++round) {
+        for (int round = 0; ok && round < 5; ++round) {
             ok = cuda_ok(cudaEventRecord(e0, st), "cudaEventRecord");
             for (int i = 0; ok && i < reps; ++i) ok = call();
             float t = 0;
@@ -563,9 +564,10 @@ uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream) {
         // Every kind of call runs the split that is set, and the kinds disagree (2^18 points,
         // R = 2^6 against 2^8: lone products 29 and 32 us, squares 33 and 23), so a split
         // has to suit them all: lone products, squares, and the members of a batch.
-        std::vector<ntt_request> members(std::min(kMaxMembers, results >> log_t));
-        for (size_t i = 0; i < members.size(); ++i)
-            members[i] = ntt_request{dst + (i << log_t), na + nb, a, b, na, nb, 0, 0, 0, 0};
+        ntt_request members[kMaxMembers];
+        const int count = (int)std::min<u64>(kMaxMembers, results >> log_t);
+        for (int i = 0; i < count; ++i)
+            members[i] = ntt_request{dst + ((u64)i << log_t), na + nb, a, b, na, nb, 0, 0, 0, 0};
         struct Times {
             float mul, sqr, batch;
         };
@@ -576,15 +578,15 @@ uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream) {
             t.sqr = log_t > kLazySquareLog ? 0.0f : time([&] {
                 return ntt_mul_workspace_sqr_device(ws, dst, na + nb, a, (u64)1 << (log_t - 1), st) == 1;
             });
-            t.batch = time([&] { return ntt_batch_run_device(batch, members.data(), members.size(), st) == 1; });
+            t.batch = time([&] { return ntt_batch_run_device(batch, members, count, st) == 1; });
             return t;
         };
         const int before = g_split[log_t].load();
         // the defaults first and last, every other split between
         Times standard = measure(0);
-        std::vector<std::pair<int, Times>> tried;
+        Times tried[kMaxLogT + 1];
         for (int r = lo; ok && r <= hi; ++r)
-            if (r != default_split(log_t)) tried.emplace_back(r, measure(r));
+            if (r != default_split(log_t)) tried[r] = measure(r);
         const Times again = measure(0);
         if (!ok) {  // a failed trial leaves the split as it was
             g_split[log_t].store(before);
@@ -595,9 +597,10 @@ uint8_t ntt_tune_splits(int min_log_t, int max_log_t, int reps, void* stream) {
         // another split only when products gain at least 2% and nothing else loses 1%
         float best = 0.98f * standard.mul;
         int pick = 0;
-        for (const auto& [r, t] : tried)
-            if (t.mul < best && t.sqr <= 1.01f * standard.sqr && t.batch <= 1.01f * standard.batch) {
-                best = t.mul;
+        for (int r = lo; r <= hi; ++r)
+            if (r != default_split(log_t) && tried[r].mul < best && tried[r].sqr <= 1.01f * standard.sqr &&
+                tried[r].batch <= 1.01f * standard.batch) {
+                best = tried[r].mul;
                 pick = r;
             }
         g_split[log_t].store(pick);
